@@ -56,7 +56,7 @@ __global__ void hv_scatter_kernel(const double *__restrict__ pts, uint32_t n, ui
             xs[ry] = p[0];
             zs[rz] = p[2];
         } else {
-            wbits[ry] = __double_as_longlong(rx - p[0]);
+            wbits[ry] = __double_as_longlong(rx == p[0] ? 0.0 : rx - p[0]); // (also where both are infinite)
         }
     }
 }
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kAreaThreads)
     for (uint32_t u = 0; u < kPer; ++u) {
         if (w[u] > run) {
             const double y = ys[p0 + u];
-            if (has) a = fma(pend_w, y - pend_y, a);
+            if (has && y != pend_y) a = fma(pend_w, y - pend_y, a); // (either side of a product may be infinite)
             if (!has) first_y = y;
             has = true;
             run = w[u];
@@ -248,6 +248,11 @@ __global__ void __launch_bounds__(kLvThreads)
     bool walking = false, done = !level;
     int v = -1, own_k = 0; // the staircase's width key so far, the own point's
     double step_x = rx, step_y = 0.0, own_x = 0.0, a = 0.0;
+    // the step up to y; one of no width or no height adds nothing, even where
+    // the other side, or both ends of this one, are infinite
+    const auto add = [&](double y) {
+        if (step_x != own_x && y != step_y) a = fma(step_x - own_x, y - step_y, a);
+    };
     int carry = -1;                  // the widest earlier point of z position below i0
     uint32_t ns = 0, q0 = 0, q1 = 0; // staircase points, own points [q0, q1) of the piece
     if (level) own_at[threadIdx.x] = INT_MAX;
@@ -413,7 +418,7 @@ __global__ void __launch_bounds__(kLvThreads)
                     x = o_x[oj];
                     y = o_y[oj];
                 }
-                if (y != step_y) a = fma(step_x - own_x, y - step_y, a);
+                add(y);
                 step_x = x;
                 step_y = y;
                 done = v > own_k;
@@ -424,10 +429,9 @@ __global__ void __launch_bounds__(kLvThreads)
     }
     double t = 0.0;
     if (level) {
-        // (a step of no height or depth adds nothing even when the other side is infinite)
-        if (!done && ry != step_y) a = fma(step_x - own_x, ry - step_y, a);
-        const double dz = rz - zs[own];
-        t = dz == 0.0 || (a == 0.0 && isinf(dz)) ? 0.0 : dz * a;
+        if (!done) add(ry);
+        const double z = zs[own];
+        t = a > 0.0 && rz != z ? (rz - z) * a : 0.0;
     }
     // the block's sum: 128 additions on this SM's FP64 pipe instead of n on hv_sum_kernel's
 #pragma unroll
