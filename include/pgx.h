@@ -138,6 +138,14 @@ PGX_API int pgx_batch_eval_device(pgx_context *ctx, int kind, uint64_t param, co
    (their callers then report PGX_ERR_TIMEOUT); the context stays usable. */
 PGX_API int pgx_selftest_barrier_timeout(pgx_context *ctx, uint64_t spin_limit, int32_t *timed_out);
 
+/* The same for the waits between the warps that find the fronts of a large
+   two-objective population (1025 .. 32768 points, host buffer of n x 2): a
+   survival pass whose waits give up after spin_limit polls. *n_fronts
+   receives what pgx_nsga2_survival_device leaves in *d_n_fronts: the number of
+   fronts, or -1 when a wait gave up (with a limit of 1 nearly all do). */
+PGX_API int pgx_selftest_front_timeout(pgx_context *ctx, const double *points, uint64_t n, uint64_t spin_limit,
+                                       int32_t *n_fronts);
+
 /* Self-test of the reciprocal and its cube in the Lennard-Jones pair loops
    (no counterpart in the reference, whose pair sum divides and cubes in FP64:
    src/problems/lennard_jones.cpp:83): inv[i] = 1/d[i] and, when inv_cube is
@@ -351,8 +359,9 @@ PGX_API int pgx_std_sort_i64(pgx_context *ctx, int64_t *keys, int32_t *values, u
 
 /* Device-resident survival: all pointers are device memory; d_n_fronts is a
    device int32. Asynchronous on `stream`. The front peeling waits on grid
-   barriers with a bounded spin (about a second); if one gives up, the call
-   still returns and *d_n_fronts reads -1 once the stream has run. */
+   barriers (for two objectives, between the warps of a cluster) with a bounded
+   spin (a second at most); if one gives up, the call still returns and
+   *d_n_fronts reads -1 once the stream has run. */
 PGX_API int pgx_nsga2_survival_device(pgx_context *ctx, const double *d_points, uint64_t n, uint64_t m, int32_t *d_rank,
                               int32_t *d_dom_count, int32_t *d_front_offsets, int32_t *d_front_indices,
                               int32_t *d_n_fronts, double *d_crowding, void *stream);
@@ -367,7 +376,7 @@ PGX_API int pgx_nsga2_survival_device(pgx_context *ctx, const double *d_points, 
    n <= 4096 and m <= 8, else PGX_ERR_CAPACITY. The first call on each device
    (and in each CUDA context) does a one-time set-up: it looks up that array's
    device address and loads the library's survival code and data on the device
-   (under lazy module loading, the CUDA default, this is when the ~2.6 MB array
+   (under lazy module loading, the CUDA default, this is when the ~2.9 MB array
    is allocated). Make that first call before another allocator reserves the
    device's memory, and before any stream capture; later calls allocate
    nothing. All calls share the array and it keeps the last call's contents

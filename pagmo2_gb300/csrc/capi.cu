@@ -629,6 +629,18 @@ int pgx_selftest_barrier_timeout(pgx_context *ctx, uint64_t spin_limit, int32_t 
     return run_barrier_timeout_test(ctx, spin_limit, timed_out);
 }
 
+int pgx_selftest_front_timeout(pgx_context *ctx, const double *points, uint64_t n, uint64_t spin_limit,
+                               int32_t *n_fronts)
+{
+    PGX_CHECK(ctx != nullptr && points != nullptr && n_fronts != nullptr, PGX_ERR_INVALID, "null argument");
+    PGX_CHECK(n > 1024u && n <= 32768u, PGX_ERR_INVALID, "number of points out of range [1025, 32768]");
+    PGX_CHECK(spin_limit >= 1u && spin_limit <= (uint64_t(1) << 24), PGX_ERR_INVALID,
+              "spin limit out of range [1, 2^24]");
+    std::lock_guard<std::mutex> g(ctx->lock);
+    PGX_TRY(use_device(ctx));
+    return run_front_timeout_test(ctx, points, static_cast<uint32_t>(n), static_cast<uint32_t>(spin_limit), n_fronts);
+}
+
 int pgx_selftest_lj_reciprocal(pgx_context *ctx, const double *d, uint64_t n, double *inv, double *inv_cube)
 {
     PGX_CHECK(ctx != nullptr && (n == 0 || (d != nullptr && inv != nullptr)), PGX_ERR_INVALID, "null argument");

@@ -2560,6 +2560,38 @@ int run_barrier_timeout_test(pgx_context *ctx, uint64_t spin_limit, int32_t *tim
     return PGX_OK;
 }
 
+// A survival pass of the two-objective kernels over host points, their waits
+// limited to spin_limit polls; *n_fronts receives what a device caller reads.
+int run_front_timeout_test(pgx_context *ctx, const double *points, uint32_t n, uint32_t spin_limit, int32_t *n_fronts)
+{
+    const size_t bp = align256(2u * static_cast<size_t>(n) * sizeof(double)), bn = align256(n * sizeof(int32_t));
+    const size_t bo = align256((static_cast<size_t>(n) + 1u) * sizeof(int32_t));
+    PGX_TRY(ctx->s_points.ensure(bp + align256(n * sizeof(double)) + 3u * bn + bo + 256u));
+    PGX_TRY(ctx->s_state.ensure(survival_scratch_bytes(n, 2u)));
+    const survival_scratch sc = carve_survival_scratch(ctx->s_state.ptr, n, 2u);
+    char *p = ctx->s_points.as<char>();
+    double *d_points = reinterpret_cast<double *>(p);
+    survival_out o{};
+    o.crowding = reinterpret_cast<double *>(p += bp);
+    o.rank = reinterpret_cast<int32_t *>(p += align256(n * sizeof(double)));
+    o.dom_count = reinterpret_cast<int32_t *>(p += bn);
+    o.front_indices = reinterpret_cast<int32_t *>(p += bn);
+    o.front_offsets = reinterpret_cast<int32_t *>(p += bn);
+    o.n_fronts = reinterpret_cast<int32_t *>(p += bo);
+    cudaStream_t s = ctx->stream;
+    PGX_CUDA(cudaMemcpyAsync(d_points, points, 2u * static_cast<size_t>(n) * sizeof(double), cudaMemcpyHostToDevice, s));
+    PGX_TRY(launch_two_survival(sc.Dt, sc.keys, sc.st, d_points, n, o, true, n, ctx->num_sms, s, &ctx->launches,
+                                spin_limit));
+    PGX_TRY(launch_front_crowding(sc, d_points, n, 2u, o.front_offsets, o.front_indices, o.n_fronts, kCrowdNsga2,
+                                  o.crowding, ctx->num_sms, s));
+    ctx->launches += crowding_launches(n, 2u);
+    int32_t h = 0;
+    PGX_CUDA(cudaMemcpyAsync(&h, o.n_fronts, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    PGX_CUDA(cudaStreamSynchronize(s));
+    *n_fronts = h;
+    return PGX_OK;
+}
+
 size_t sort_pairs_state_bytes()
 {
     return sizeof(peel_state);

@@ -189,7 +189,9 @@ __device__ __forceinline__ uint32_t two_block_scan(uint32_t v, uint32_t *part, u
 // minimum of kTwoInf says that no earlier warp has points left, now or later.
 // Messages go through a ring of kTwoRing words per warp in its block's shared
 // memory, (k + 1) << 16 | minimum, so that a word tells whose it is; the
-// receiver acknowledges every half ring. Waits are bounded (st->err).
+// receiver acknowledges every half ring. Waits are bounded by spin_limit polls;
+// when one runs out, those behind it do too, st->err is set and the number of
+// fronts is -1, for which the kernels after this one do nothing.
 // n = 20000, 153 fronts: 112 us, some 1400 cycles a front for the slowest warp
 // (one block with barriers, 20 positions per thread: 220 us; rows behind
 // branches on their number, not interleaved: 168 us).
@@ -232,7 +234,7 @@ __device__ __forceinline__ void two_cluster_sync()
 // Q: registers of two rows each.
 template <uint32_t Q>
 __global__ void __cluster_dims__(kTwoBlocks, 1, 1) __launch_bounds__(kTwoWarps * 32, 1)
-    two_peel_kernel(two_scratch s, uint32_t n, int32_t *__restrict__ n_fronts, peel_state *st)
+    two_peel_kernel(two_scratch s, uint32_t n, uint32_t spin_limit, int32_t *__restrict__ n_fronts, peel_state *st)
 {
     chain_wait();
     __shared__ uint32_t ring[kTwoWarps][kTwoRing], acked[kTwoWarps];
@@ -286,7 +288,7 @@ __global__ void __cluster_dims__(kTwoBlocks, 1, 1) __launch_bounds__(kTwoWarps *
             if (waiting) {
                 const uint32_t *slot = ring[warp] + k % kTwoRing;
                 uint32_t m = two_peek(slot), spins = 0;
-                while (m >> 16 != k + 1u && ++spins < kTwoSpins) m = two_peek(slot);
+                while (m >> 16 != k + 1u && ++spins < spin_limit) m = two_peek(slot);
                 m = __shfl_sync(kFull, m, 0); // (lanes may have read it at different times)
                 if (m >> 16 != k + 1u) {
                     failed = true;
@@ -300,7 +302,7 @@ __global__ void __cluster_dims__(kTwoBlocks, 1, 1) __launch_bounds__(kTwoWarps *
             if (!last) {
                 if (k >= room) {
                     uint32_t a = two_peek(acked + warp), spins = 0;
-                    while (k >= a + kTwoRing && ++spins < kTwoSpins) a = two_peek(acked + warp);
+                    while (k >= a + kTwoRing && ++spins < spin_limit) a = two_peek(acked + warp);
                     a = __shfl_sync(kFull, a, 0);
                     if (k >= a + kTwoRing) {
                         failed = true;
@@ -329,11 +331,17 @@ __global__ void __cluster_dims__(kTwoBlocks, 1, 1) __launch_bounds__(kTwoWarps *
         }
         if (failed && lane == 0u) st->err = 1;
         if (last && lane == 0u) {
-            *n_fronts = failed ? 0 : static_cast<int32_t>(k);
-            st->n_fronts = failed ? 0 : static_cast<int32_t>(k);
+            *n_fronts = failed ? -1 : static_cast<int32_t>(k);
+            st->n_fronts = failed ? -1 : static_cast<int32_t>(k);
         }
     }
     two_cluster_sync(); // no block leaves while its shared memory may be written
+}
+
+// The number of fronts; 0, and nothing to do, where the waits ran out.
+__device__ __forceinline__ uint32_t two_fronts(const int32_t *n_fronts)
+{
+    return static_cast<uint32_t>(max(*n_fronts, 0));
 }
 
 // The fronts' offsets and unordered lists of positions, written out in order
@@ -352,8 +360,8 @@ __global__ void __launch_bounds__(kTwoThreads, 1)
     __shared__ uint32_t part[32];
     uint32_t *cnt = reinterpret_cast<uint32_t *>(two_mem);
     uint16_t *mem = reinterpret_cast<uint16_t *>(two_mem + align256(n * sizeof(uint32_t)));
-    const uint32_t tid = threadIdx.x, F = static_cast<uint32_t>(*n_fronts);
-    if (F == 0u) return; // (the fronts' waits ran out)
+    const uint32_t tid = threadIdx.x, F = two_fronts(n_fronts);
+    if (F == 0u) return;
     for (uint32_t f = tid; f < F; f += kTwoThreads) cnt[f] = 0u;
     constexpr uint32_t kPer = kTwoPoints / kTwoThreads;
     uint32_t of[kPer];
@@ -452,7 +460,7 @@ __global__ void __launch_bounds__(kStairThreads)
 {
     chain_wait();
     __shared__ uint32_t list[kStairWords], before[kStairWords], part[32];
-    const uint32_t F = static_cast<uint32_t>(*n_fronts);
+    const uint32_t F = two_fronts(n_fronts);
     for (uint32_t x = blockIdx.x; x < 2u * F; x += gridDim.x) {
         const uint32_t f = x >> 1, off = static_cast<uint32_t>(front_offsets[f]);
         const uint32_t L = static_cast<uint32_t>(front_offsets[f + 1u]) - off;
@@ -494,7 +502,7 @@ __global__ void two_ranges_kernel(two_scratch s, uint32_t n, const int32_t *__re
                                   const int32_t *__restrict__ n_fronts)
 {
     chain_wait();
-    if (*n_fronts == 0) return; // (the fronts' waits ran out)
+    if (two_fronts(n_fronts) == 0u) return;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint32_t p = static_cast<uint32_t>(s.order[t]), u = static_cast<uint32_t>(s.uq[p]);
         const int32_t f = s.rank_u[u];
@@ -805,7 +813,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1)
     uint32_t *comp = reinterpret_cast<uint32_t *>(two_mem);
     uint16_t *high = reinterpret_cast<uint16_t *>(two_mem + align256(two_skew(two_order_room(n)) * sizeof(uint32_t)));
     const two_high run{high, by8, by64, by512};
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, F = static_cast<uint32_t>(*n_fronts);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, F = two_fronts(n_fronts);
     uint32_t K = 1u; // positions of the front before
     cnt[tid] = 0u;
     if (tid == 0u) many = 0;
@@ -1039,7 +1047,7 @@ bool two_fits(uint32_t n, uint32_t m)
 // base: two_scratch_bytes(n).
 int launch_two_survival(void *base, long long *keys, peel_state *st, const double *pts, uint32_t n,
                         const survival_out &out, bool counts, uint32_t need, int num_sms, cudaStream_t s,
-                        uint64_t *launches)
+                        uint64_t *launches, uint32_t spin_limit = kTwoSpins)
 {
     const two_scratch sc = carve_two_scratch(base, n);
     const int pl = launch_positions(pts, n, 2u, 0u, 2u, sc.runs, sc.pos, num_sms, s);
@@ -1061,7 +1069,7 @@ int launch_two_survival(void *base, long long *keys, peel_state *st, const doubl
                       : q == 3u ? two_peel_kernel<3>
                                 : two_peel_kernel<4>;
     static_assert(kTwoRows == 8u, "four registers hold a warp's rows");
-    PGX_CUDA(launch_chained(peel, kTwoBlocks, kTwoWarps * 32, 0, s, sc, n, out.n_fronts, st));
+    PGX_CUDA(launch_chained(peel, kTwoBlocks, kTwoWarps * 32, 0, s, sc, n, spin_limit, out.n_fronts, st));
     PGX_CUDA(cudaFuncSetAttribute(two_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(two_lists_smem(kTwoPoints))));
     PGX_CUDA(launch_chained(two_lists_kernel, 1, kTwoThreads, two_lists_smem(n), s, sc, n, out.front_offsets,
