@@ -610,11 +610,11 @@ int build_plan(pgx_epoch *ep, const pgx_request *reqs, int n_reqs)
     const auto shared_of = [&](int w) {
         return (ep->sm_table + static_cast<size_t>(ep->sm_per_warp) * static_cast<size_t>(w)) * sizeof(double);
     };
-    constexpr size_t kMostShared = 227u * 1024u;
     const bool wide_fits = shared_of(kWideWarps) <= kMostShared;
-    PGX_CUDA(cudaFuncSetAttribute(
-        epoch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        static_cast<int>(std::max<size_t>(shared_of(wide_fits ? kWideWarps : kWarpsPerBlock), 48u * 1024u))));
+    // the limit is the kernel's, not the plan's: the same for every plan, or one
+    // made later would lower it below what an earlier one launches with
+    PGX_CUDA(cudaFuncSetAttribute(epoch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kMostShared)));
     int occ = 0, occ_wide = 0;
     PGX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, epoch_kernel, kWarpsPerBlock * 32,
                                                            shared_of(kWarpsPerBlock)));

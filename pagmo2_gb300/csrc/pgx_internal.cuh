@@ -78,6 +78,12 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// The most shared memory that a block may ask for on GB300. A kernel's limit
+// (cudaFuncAttributeMaxDynamicSharedMemorySize) is one for all contexts and
+// threads of a device, so it is always set to the same value, never to one
+// call's need.
+constexpr size_t kMostShared = 227u * 1024u;
+
 // --------------------------------------------------------- device buffers
 
 // Grow-only device allocation owned by a context.
