@@ -284,8 +284,7 @@ int launch_lj(K kernel, bool grad, const double *x, uint64_t n, uint32_t na, uin
     if (wpb < 1) wpb = 1;
     const int threads = 32 * wpb;
     const size_t smem = per_warp * wpb;
-    PGX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem > 48u * 1024u ? smem : 48u * 1024u)));
+    PGX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMostShared)));
     int grid = 1;
     PGX_TRY(grid_for(kernel, threads, smem, n, wpb, num_sms, &grid));
     PGX_CUDA(launch_chained(kernel, grid, threads, smem, s, x, n, na, nx, f, g));

@@ -210,8 +210,9 @@ int launch_refine_kernel(K kernel, int lanes, size_t smem_per_warp, const refine
     }
     const int threads = 32 * warps;
     const size_t smem = smem_per_warp * static_cast<size_t>(warps);
-    PGX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem > 48u * 1024u ? smem : 48u * 1024u)));
+    if (smem) // (clusters' kernels, which have no other shared memory)
+        PGX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kMostShared)));
     int occ = 0;
     PGX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
     if (occ < 1) occ = 1;

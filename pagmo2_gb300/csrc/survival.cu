@@ -2218,8 +2218,10 @@ int run_survival(const survival_scratch &sc, const double *d_points, uint32_t n,
                        + (n <= kPosPoints ? static_cast<size_t>(W) * 4u + 2u * ((static_cast<size_t>(n) * 2u + 3u) & ~size_t(3))
                                           : 0u);
         if (fused) smem2 = std::max(smem2, kSortSmemBytes);
+        cudaFuncAttributes peel2_is{};
+        PGX_CUDA(cudaFuncGetAttributes(&peel2_is, peel2_kernel));
         PGX_CUDA(cudaFuncSetAttribute(peel2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem2)));
+                                      static_cast<int>(kMostShared - peel2_is.sharedSizeBytes)));
         int occ2 = 0;
         PGX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, peel2_kernel, kPeelThreads, smem2));
         PGX_CHECK(occ2 >= 1, PGX_ERR_CUDA, "peel kernel cannot be resident");

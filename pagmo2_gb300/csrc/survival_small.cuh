@@ -145,7 +145,7 @@ constexpr int small_threads(uint32_t n)
     return n <= 512u ? 512 : kSmallThreads;
 }
 
-constexpr size_t small_smem(uint32_t n, uint32_t m, bool crowd)
+constexpr size_t small_smem(uint32_t n, uint32_t m, bool crowd) // grows with n
 {
     const size_t keys = align256(static_cast<size_t>(n) * m * sizeof(long long));
     const size_t matrix = align256(static_cast<size_t>(n) * small_row_words(n) * sizeof(uint32_t));
@@ -441,8 +441,11 @@ int launch_small_survival_mm(small_args a, uint32_t *Dt, cudaStream_t s, uint64_
         a.Dt = Dt;
         ++*launches;
     }
+    // one limit for all calls: other contexts' threads launch the kernel at the same time
+    constexpr uint32_t most_m = MM > 0 ? static_cast<uint32_t>(MM) : kSmallObjectives;
+    constexpr size_t all = small_smem(kSmallPoints, most_m, false), inside = small_smem(kSmallCrowd, most_m, true);
     PGX_CUDA(cudaFuncSetAttribute(small_survival_kernel<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
+                                  static_cast<int>(all > inside ? all : inside)));
     PGX_CUDA(launch_chained(small_survival_kernel<MM>, 1, small_threads(a.n), smem, s, a));
     ++*launches;
     return PGX_OK;
