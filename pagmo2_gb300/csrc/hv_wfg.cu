@@ -516,9 +516,20 @@ __device__ __forceinline__ uint32_t first_dims(const wfg_args<P> &a)
     return a.contributions ? a.m : a.m - 1u; // coordinates of the items' frames
 }
 
+// The rows of level l from row0 to the list's end belong to no frame: the one
+// that would have begun there does not fit (and none after it does). Unmarked
+// they would hold what an earlier call left, whose ranks are no indexes into
+// this call's table.
+constexpr uint32_t kNoParent = 0xffffffffu;
+
+template <class P>
+__device__ __forceinline__ void mark_gap(const wfg_level<P> &L, unsigned long long row0, uint32_t t, uint32_t threads)
+{
+    for (unsigned long long g = row0 + t; g < L.row_cap; g += threads) L.row_parent[g] = kNoParent;
+}
+
 // Row g of level l when it belongs to a frame stored at that level: its frame's
-// rows k, first row off and index j; false for rows of a frame past the
-// list's end (never written: any values).
+// rows k, first row off and index j; false for marked rows.
 template <class P>
 __device__ __forceinline__ bool row_of(const wfg_args<P> &a, int l, unsigned long long g, uint32_t *k,
                                        unsigned long long *off)
@@ -542,7 +553,10 @@ __device__ bool store_frame(const wfg_args<P> &a, int l, uint64_t parent, const 
     unsigned long long row0 = 0;
     if (lane == 0) row0 = atomicAdd(L.rows_used, static_cast<unsigned long long>(k));
     row0 = __shfl_sync(kMask, row0, 0);
-    if (row0 + k > L.row_cap) return false;
+    if (row0 + k > L.row_cap) {
+        mark_gap<P>(L, row0, lane, 32u);
+        return false;
+    }
     sort_rows<P>(buf, k, d, false, L.frames + row0 * P::words(d), lane);
     for (uint32_t t = lane; t < k; t += 32u) L.row_parent[row0 + t] = static_cast<uint32_t>(parent);
     if (lane == 0) {
@@ -740,6 +754,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) wfg_top_kernel(wfg_args<P
                 }
                 continue;
             }
+            mark_gap<P>(L, row0, threadIdx.x, blockDim.x);
         }
         if (warp != 0u) continue;
         const int in = frame == base ? 0 : 1;
