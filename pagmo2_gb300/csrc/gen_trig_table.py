@@ -20,6 +20,11 @@ print("namespace pgx\n{\nnamespace trigtab\n{\n")
 print(f"constexpr int kLogN = {LOG_N};")
 print("// sin and 1 - cos of t a, a = pi / N, as polynomials in z = t^2 (Taylor coefficients: |t a| <= 0.0031, the first")
 print("// dropped terms are below 2^-75 and 2^-82)")
+a1 = q(a ** 3 / 6, 73)
+low = (a1 + 2 ** 31) % 2 ** 32 - 2 ** 31
+print(f"constexpr int64_t kFineA0 = {q(a, 67)}LL;          // a, Q67")
+print(f"constexpr int32_t kFineA1High = {(a1 - low) >> 32}, kFineA1Low = {low}; // a^3 / 6, Q73, in signed words")
+print(f"constexpr uint32_t kFineA2 = {q(a ** 5 / 120, 74)}u;             // a^5 / 120, Q74")
 print(f"constexpr int64_t kA0 = {q(a, 67) - 280}LL;              // a, Q67, less what the floored products below it take too little")
 print(f"constexpr uint32_t kA1 = {q(a ** 3 / 6, 59)}u;               // a^3 / 6, Q59")
 print(f"constexpr uint32_t kA2 = {q(a ** 5 / 120, 60)}u;                     // a^5 / 120, Q60")
