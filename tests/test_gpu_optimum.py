@@ -59,3 +59,18 @@ def test_rastrigin_refined(ctx, dim):
 def test_griewank(ctx, dim):
     f = P.from_kind(N.GRIEWANK, dim, ctx).batch_fitness(small_rows(dim))
     assert np.all(f[:3] == 0.0)
+
+
+@pytest.mark.parametrize("dim", DIMS)
+@pytest.mark.parametrize("e", [-300, -40, -30, -26, -20, -17, -16, -15])
+def test_griewank_next_to_zero(ctx, dim, e):
+    # |x| around 2^e, over the end of the table's range (2^-16), some elements 0: three roundings next to 1 (2^-54 each)
+    # and three units of 2^-62 per factor; nowhere below 0
+    rng = np.random.default_rng(dim - e)
+    x = np.ldexp(rng.uniform(0.25, 1.0, (200, dim)), e + 1) * rng.choice([-1.0, 0.0, 1.0], (200, dim), p=[0.45, 0.1, 0.45])
+    f = P.from_kind(N.GRIEWANK, dim, ctx).batch_fitness(x)
+    z = np.longdouble(1) * x * x
+    k = np.arange(1, dim + 1) * np.longdouble(1)
+    want = z.sum(axis=1) / 4000 - np.expm1(np.log1p(-(z / k / 2 - (z / k) ** 2 / 24)).sum(axis=1))
+    assert np.all(f >= 0.0)
+    assert np.all(np.abs(f - want) <= 3 * 2.0 ** -54 + 3 * dim * 2.0 ** -62 + np.abs(want) * 2.0 ** -52)
