@@ -792,7 +792,6 @@ struct peel2_args {
     // compute the crowding distances of the fronts of up to kSortSmemCap
     // members as the peel completes them (longer fronts: big_crowding_kernel)
     uint32_t npeel;
-    const double *pts;
     uint32_t m;
     const long long *keys;
     double *cd;
@@ -1411,7 +1410,7 @@ __global__ void __launch_bounds__(kPeelThreads) peel2_kernel(peel2_args a)
 // Crowding distance of every point within its front: blocks take fronts
 // f = blockIdx.x, blockIdx.x + gridDim.x, ... (n_fronts read on the device).
 __global__ void __launch_bounds__(kSortThreads) front_crowding_kernel(
-    const double *__restrict__ pts, uint32_t n, uint32_t m, const long long *__restrict__ keys,
+    uint32_t n, uint32_t m, const long long *__restrict__ keys,
     const int32_t *__restrict__ front_offsets, const int32_t *__restrict__ front_indices,
     const int32_t *__restrict__ n_fronts, int mode, unsigned char *wkey, int32_t *widx, int2 *wlist, int32_t *wpos,
     double *cd, peel_state *st)
@@ -1680,7 +1679,7 @@ __global__ void __launch_bounds__(kGridSortThreads) sort_population_big_kernel(
 // critical front's members by descending crowding distance (std::sort of the
 // positions 0..L-1 with greater_than_f, ties in std::sort's order).
 __global__ void __launch_bounds__(kSortThreads) select_best_kernel(
-    const double *__restrict__ pts, uint32_t n, uint32_t m, uint32_t N, const long long *__restrict__ keys,
+    uint32_t n, uint32_t m, uint32_t N, const long long *__restrict__ keys,
     const int32_t *__restrict__ front_offsets, const int32_t *__restrict__ front_indices,
     const int32_t *__restrict__ n_fronts, unsigned char *wkey, int32_t *widx, int2 *wlist, int32_t *wpos, double *wcd,
     int32_t *out,
@@ -2145,7 +2144,7 @@ int launch_front_crowding(const survival_scratch &sc, const double *d_points, ui
     PGX_CUDA(cudaFuncSetAttribute(front_crowding_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(kSortSmemBytes)));
     const int grid = static_cast<int>(std::min<uint64_t>(n, static_cast<uint64_t>(num_sms) * 2u));
-    PGX_CUDA(launch_chained(front_crowding_kernel, grid, kSortThreads, kSortSmemBytes, s, d_points, n, m, sc.keys, front_offsets,
+    PGX_CUDA(launch_chained(front_crowding_kernel, grid, kSortThreads, kSortSmemBytes, s, n, m, sc.keys, front_offsets,
                                                                      front_indices, n_fronts, mode, sc.wkey, sc.widx,
                                                                      sc.wlist, sc.wpos, cd, sc.st));
     if (n > static_cast<uint32_t>(kSortSmemCap) && m >= 2u) {
@@ -2238,7 +2237,7 @@ int run_survival(const survival_scratch &sc, const double *d_points, uint32_t n,
         }
         *launches += 2;
         peel2_args pa{sc.Dt, out.dom_count, n, W, W8, sc.wit, sc.widx, sc.list, sc.keyv, sc.cnt,
-                      out.rank, out.front_offsets, out.front_indices, sc.st, npeel, d_points, m, sc.keys,
+                      out.rank, out.front_offsets, out.front_indices, sc.st, npeel, m, sc.keys,
                       fused ? out.crowding : nullptr, kCrowdNsga2};
         void *args2[] = {&pa};
         PGX_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(peel2_kernel), dim3(num_sms),
@@ -2495,7 +2494,7 @@ int launch_select_best(pgx_context *ctx, const double *d_points, uint64_t n64, u
     PGX_TRY(run_survival(sc, d_points, n, m, fb.o, false, N, sms, s, &ctx->launches));
     PGX_CUDA(cudaFuncSetAttribute(select_best_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(kSortSmemBytes)));
-    PGX_CUDA(launch_chained(select_best_kernel, 1, kSortThreads, kSortSmemBytes, s, d_points, n, m, N, sc.keys, fb.o.front_offsets,
+    PGX_CUDA(launch_chained(select_best_kernel, 1, kSortThreads, kSortSmemBytes, s, n, m, N, sc.keys, fb.o.front_offsets,
                                                                fb.o.front_indices, fb.o.n_fronts, sc.wkey, sc.widx,
                                                                sc.wlist, sc.wpos, sc.wcd, d_out, sc.st));
     ++ctx->launches;

@@ -8,15 +8,16 @@
 // The matrix and the keys are in shared memory (n = 1024, m = 8: 196 KB); the
 // sort areas of the crowding step reuse the matrix's room. Beyond
 // kSmallOwnMatrix points the pair tests, n^2 / 2 on one SM otherwise (1000 x 3:
-// 100 us), come from a kernel on all of them before. Short fronts are sorted by
-// one warp each, all at the same time, longer ones by the whole block one after
-// the other.
+// 100 us), come from a kernel on all of them before. Up to kSmallCrowd points the
+// block sorts the fronts too: short ones by one warp each, all at the same time,
+// the one that may be longer by the whole block; beyond, front_crowding_kernel
+// gives each front a block.
 //
 // What bounds it: dependent instructions of few warps, in the exact sorts of
 // the crowding (700 cycles per partition of 17 to 33 members) and in the peel
-// (2700 cycles per front). 200 x 2 points: 12 layers 135 -> 26 us, one 73 -> 31;
-// 512 x 3: 100 -> 65; 1000 x 3: 118 -> 108, 1024 x 2 in 40 layers 276 -> 120.
-// Beyond kSmallPoints a block has no thread per point.
+// (2700 cycles per front). By the general pass and now, us: 200 x 2 points in 12
+// layers 135, 30, in one 84, 31; 512 x 3 in 10 114, 68; 1000 x 3 in 10 134, 94;
+// 1024 x 2 in 40 278, 114. Beyond kSmallPoints a block has no thread per point.
 #pragma once
 
 namespace pgx
@@ -27,10 +28,10 @@ namespace
 constexpr uint32_t kSmallPoints = 1024;
 constexpr uint32_t kSmallObjectives = 8;
 constexpr int kSmallThreads = 1024;
-// Longest front one warp sorts: the block is quicker on a single front of more
-// than kOneWarpFront members (one of 200: 31 against 40 us in all), the warps on
-// several at once (eight of 125 and more: 108 against 254 us).
-constexpr int kOneWarpFront = 128, kWarpFront = 256;
+// Longest front one warp sorts: the block is quicker on one of more than
+// kOneWarpFront members (one of 200: 31 against 40 us in all), and no two of
+// these fit into the kSmallCrowd points that the block sorts at all.
+constexpr int kOneWarpFront = 128;
 
 // The sort arrays of all fronts, by position in front order: a front works in
 // its own slice, whichever warp takes it.
@@ -42,9 +43,10 @@ struct warp_sort_area {
                        // as ranges of at most 16 never wait
 };
 
-// std::sort's permutation (introsort.cuh) of x[0 .. n), n <= kWarpFront, by one
+// std::sort's permutation (introsort.cuh) of x[0 .. n), n <= kOneWarpFront, by one
 // warp: the ranges longer than 16 one after the other from a stack (they are
-// disjoint, so at most kWarpFront / 17 wait), the shorter ones as they appear.
+// disjoint, so at most kOneWarpFront / 17 wait), the shorter ones as they appear.
+static_assert(kOneWarpFront <= dev::kShortRange, "the warp's partitions are short ones");
 __device__ void warp_std_sort(const dev::sort_view<long long> &x, int n, const dev::sort_work &w, int *stack, int *err)
 {
     const unsigned lane = threadIdx.x & 31u;
@@ -58,8 +60,7 @@ __device__ void warp_std_sort(const dev::sort_view<long long> &x, int n, const d
             if (lane == 0) dev::heap_sort(x, first, last);
             __syncwarp();
         } else {
-            const int cut = last - first <= dev::kShortRange ? dev::warp_partition_short(x, first, last, w, err)
-                                                              : dev::warp_partition(x, first, last, w, err);
+            const int cut = dev::warp_partition_short(x, first, last, w, err);
             const int la = lane < 16u ? first : cut, len = lane < 16u ? cut - first : last - cut;
             dev::halfwarp_leaf_sort(x, la, len <= 16 ? len : 0);
             --depth;
@@ -93,7 +94,7 @@ __device__ void warp_std_sort(const dev::sort_view<long long> &x, int n, const d
     }
 }
 
-// front_crowding for a front of 2 <= L <= kWarpFront members by one warp, the
+// front_crowding for a front of 2 <= L <= kOneWarpFront members by one warp, the
 // distances into s_cd (by point).
 __device__ void warp_front_crowding(uint32_t n, uint32_t m, const long long *keys, const uint16_t *members, int L,
                                     const warp_sort_area &a, int *err, double *s_cd)
@@ -383,18 +384,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_survival_kernel(small_
     // ---- crowding (the matrix's room is free)
     long long *ak = reinterpret_cast<long long *>(area);
     int *ai = reinterpret_cast<int *>(ak + n);
-    int longer = 0; // fronts longer than kOneWarpFront
-    for (int f0 = 0; f0 < k; f0 += static_cast<int>(blockDim.x)) {
-        const int f = f0 + static_cast<int>(threadIdx.x);
-        longer += __syncthreads_count(f < k && s_off[f + 1] - s_off[f] > kOneWarpFront);
-    }
-    const int by_warp = longer > 1 ? kWarpFront : kOneWarpFront;
     for (int f = static_cast<int>(warp); f < k; f += static_cast<int>(nwarps)) {
         const int L = s_off[f + 1] - s_off[f];
         const uint16_t *mem = s_front + s_off[f];
         if (L == 1 || (L == 2 && a.crowd_mode == kCrowdNsga2)) {
             if (static_cast<int>(lane) < L) s_cd[mem[lane]] = a.crowd_mode == kCrowdNsga2 ? HUGE_VAL : 0.0;
-        } else if (L <= by_warp) {
+        } else if (L <= kOneWarpFront) {
             const int at = s_off[f];
             const warp_sort_area mine{ak + at, ai + at, ai + n + at, ai + 2u * n + at, ai + 3u * n + 3 * (at / 16)};
             warp_front_crowding(n, m, keys, mem, L, mine, &a.st->sort_err, s_cd);
@@ -403,7 +398,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_survival_kernel(small_
     __syncthreads();
     for (int f = 0; f < k; ++f) {
         const int L = s_off[f + 1] - s_off[f];
-        if (L <= by_warp) continue; // uniform: the same front for every thread
+        if (L <= kOneWarpFront) continue; // uniform: the same front for every thread
         const sort_area<long long> sa = pick_area<long long>(area, L, nullptr, nullptr, nullptr, nullptr);
         front_crowding(n, m, keys, a.front_indices + s_off[f], L, sa, &ctl, slots, &a.st->sort_err, s_cd);
     }
