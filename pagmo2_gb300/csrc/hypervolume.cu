@@ -20,6 +20,7 @@
 // a tie does not change any slab (its step is zero). The widths r_x - x are
 // non-negative on valid input, so their running maximum is taken on integers:
 // the IEEE bit patterns (2D) or the reversed x positions (3D).
+#include "fitness_dev.cuh"
 #include "sort_pos.cuh"
 #include "pgx_internal.cuh"
 
@@ -442,26 +443,33 @@ __global__ void __launch_bounds__(kLvThreads)
     if (threadIdx.x == 0) term[blockIdx.x] = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
 }
 
-// out = sum of term[0 .. L) in a fixed tree (one block; the partial sums of
-// the blocks before it: few, because one SM adds only 2 doubles per clock)
+// out = sum of term[0 .. L), none negative, by one block: an integer sum
+// (isum.h: within 2^-60 per addition, rounded once), as the last additions of a
+// tree of doubles, each rounded at the volume's own size, were most of its error.
 constexpr int kHvSumThreads = 256;
 
 __global__ void __launch_bounds__(kHvSumThreads) hv_sum_kernel(const double *__restrict__ term, uint32_t L,
                                                                double *__restrict__ out)
 {
     chain_wait();
-    __shared__ double part[kHvSumThreads / 32];
-    double s = 0.0;
-    for (uint32_t i = threadIdx.x; i < L; i += kHvSumThreads) s += term[i];
-#pragma unroll
-    for (int h = 16; h > 0; h >>= 1) s += __shfl_down_sync(kFull, s, h);
-    if ((threadIdx.x & 31u) == 0u) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s = part[0];
-        for (int q = 1; q < kHvSumThreads / 32; ++q) s += part[q];
-        *out = s;
+    __shared__ unsigned long long part_m[kHvSumThreads / 32];
+    __shared__ int part_e[kHvSumThreads / 32];
+    __shared__ uint32_t part_flags[kHvSumThreads / 32];
+    isum::sq_acc s = isum::make();
+    for (uint32_t i = threadIdx.x; i < L; i += kHvSumThreads) isum::add(s, isum::magnitude(term[i], s.flags));
+    s = dev::group_isum<32>(s, kFull);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0u) {
+        part_m[warp] = s.m;
+        part_e[warp] = s.e;
+        part_flags[warp] = s.flags;
     }
+    __syncthreads();
+    if (warp != 0u) return;
+    const bool has = lane < kHvSumThreads / 32;
+    s = has ? isum::sq_acc{part_m[lane], part_e[lane], part_flags[lane]} : isum::make();
+    s = dev::group_isum<32>(s, kFull);
+    if (lane == 0u) *out = isum::value(s);
 }
 
 // hypervolume::verify_after_construct and verify_before_compute with
