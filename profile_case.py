@@ -14,9 +14,9 @@ profiler are not benchmark values). Cases:
   ackley_f / griewank_f / schwefel_f   dim 50 (--dim), fitness only
   zdt<k>_f                      ZDT k, param 30 (--dim), objectives n x 2
   dtlz<k>_f                     DTLZ k, dim 12 (--dim), 3 objectives (--fdim)
-  survival                      NSGA-II survival of --rows nested-front points x 3
-  select_best                   select_best_N_mo(--rows nested-front points x 3, rows / 2)
-  sort_population               sort_population_mo(--rows nested-front points x 3)
+  survival                      NSGA-II survival of --rows nested-front points x --fdim (default 3)
+  select_best                   select_best_N_mo(--rows nested-front points x --fdim, rows / 2)
+  sort_population               sort_population_mo(--rows nested-front points x --fdim)
   hypervolume                   hypervolume of --rows nested-front points x 3 (reference point max + 0.5)
   hv_wfg / hv_contributions     hypervolume / every point's contribution of --rows points on a sphere front of
                                 --fdim objectives (default 5; reference point 1.1)
@@ -43,7 +43,7 @@ def main() -> None:
     ap.add_argument("--launches", type=int, default=3)
     ap.add_argument("--atoms", type=int, default=150, help="lennard_jones cluster size (lj_* cases)")
     ap.add_argument("--dim", type=int, default=0, help="rastrigin/rosenbrock dimension (default 50 / 1000)")
-    ap.add_argument("--fdim", type=int, default=3, help="DTLZ objectives (dtlz* cases)")
+    ap.add_argument("--fdim", type=int, default=3, help="objectives (dtlz*, survival, select_best and sort_population)")
     ap.add_argument("--layers", type=int, default=30, help="nested fronts of the survival/select_best/sort cases")
     a = ap.parse_args()
 
@@ -86,14 +86,14 @@ def main() -> None:
             N.check(L.pgx_refine_batch_device(ctx.handle, kind, param, C.byref(params), dx.data_ptr(), n,
                                               df.data_ptr(), de.data_ptr(), sp))
     elif a.case == "survival":
-        p = W.nsga2_points(n, 3, layers=a.layers)
+        p = W.nsga2_points(n, a.fdim, layers=a.layers)
         dp = torch.from_numpy(p).cuda()
         i32 = lambda k: torch.empty(k, dtype=torch.int32, device="cuda")  # noqa: E731
         rank, dc, off, idx, nf = i32(n), i32(n), i32(n + 1), i32(n), i32(1)
         cd = torch.empty(n, dtype=torch.float64, device="cuda")
 
         def run():
-            N.check(L.pgx_nsga2_survival_device(ctx.handle, dp.data_ptr(), n, 3, rank.data_ptr(), dc.data_ptr(),
+            N.check(L.pgx_nsga2_survival_device(ctx.handle, dp.data_ptr(), n, a.fdim, rank.data_ptr(), dc.data_ptr(),
                                                 off.data_ptr(), idx.data_ptr(), nf.data_ptr(), cd.data_ptr(), sp))
     elif a.case == "hypervolume":
         p = W.nsga2_points(n, 3, layers=a.layers)
@@ -117,17 +117,17 @@ def main() -> None:
                 N.check(L.pgx_hypervolume_contributions_device(ctx.handle, dp.data_ptr(), n, m, N.ptr(r),
                                                                dout.data_ptr(), sp))
     elif a.case in ("select_best", "sort_population"):
-        p = W.nsga2_points(n, 3, layers=a.layers)
+        p = W.nsga2_points(n, a.fdim, layers=a.layers)
         dp = torch.from_numpy(p).cuda()
         sel = torch.empty(n, dtype=torch.int32, device="cuda")
         st = torch.empty(1, dtype=torch.int32, device="cuda")
 
         def run():
             if a.case == "select_best":
-                N.check(L.pgx_select_best_n_mo_device(ctx.handle, dp.data_ptr(), n, 3, n // 2, sel.data_ptr(),
+                N.check(L.pgx_select_best_n_mo_device(ctx.handle, dp.data_ptr(), n, a.fdim, n // 2, sel.data_ptr(),
                                                       st.data_ptr(), sp))
             else:
-                N.check(L.pgx_sort_population_mo_device(ctx.handle, dp.data_ptr(), n, 3, sel.data_ptr(),
+                N.check(L.pgx_sort_population_mo_device(ctx.handle, dp.data_ptr(), n, a.fdim, sel.data_ptr(),
                                                         st.data_ptr(), sp))
     elif a.case.startswith(("zdt", "dtlz")):
         import ctypes as C
