@@ -63,7 +63,7 @@ constexpr uint32_t kGriewankColumns = 1024;
 // `batch` rows one after the other (1, or G), and each lane then closes one of
 // them: with one row at a time only one lane in G works on the closing
 // expression, half of ackley's FP64 time at 4 lanes. 1 M x 50 with the table's cosines:
-// ackley 819 -> 404 us, griewank 2930 -> 349, schwefel 2850 -> 471.
+// ackley 819 -> 408 us, griewank 2930 -> 344, schwefel 2850 -> 474.
 template <int G, int KIND>
 __global__ void __launch_bounds__(256) row_f_kernel(const double *__restrict__ x, uint64_t n, uint32_t nx,
                                                     double *__restrict__ f, uint32_t batch)
