@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kLvThreads)
     if (level) {
         if (!done) add(ry);
         const double z = zs[own];
-        t = a > 0.0 && rz != z ? (rz - z) * a : 0.0;
+        t = a != 0.0 && rz != z ? (rz - z) * a : 0.0;
     }
     // the block's sum: 128 additions on this SM's FP64 pipe instead of n on hv_sum_kernel's
 #pragma unroll
